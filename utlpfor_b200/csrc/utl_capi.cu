@@ -1042,8 +1042,8 @@ int utl_index_stream(const uint8_t* d_packed, size_t packed_len, uint64_t* d_blo
   if (rc != UTL_OK) return rc;
   UTL_CUDA(c->index.ensure(launch::index_scratch_bytes(packed_len)));
   cudaError_t ce = cudaSuccess;
-  rc = launch::index_stream(d_packed, packed_len, d_block_off, max_blocks, n_blocks, c->index.p, (cudaStream_t)stream,
-                            &ce);
+  rc = launch::index_stream(d_packed, packed_len, d_block_off, max_blocks, n_blocks, c->index.p, c->res_d(), c->res_h(),
+                            (cudaStream_t)stream, &ce);
   if (rc < 0) return cuda_fail(ce);
   return rc;
 }

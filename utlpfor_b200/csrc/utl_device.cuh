@@ -185,7 +185,7 @@ __device__ __forceinline__ void warp_exc_counts(const uint32_t w[4], const bool 
 // The block is written at byte offset dst of sm; hb is a 128-word per-warp
 // scratch.  Returns the block length (warp-uniform).
 // ---------------------------------------------------------------------------
-__device__ int warp_pack_block(const uint32_t v[4], int n, int flag, uint32_t type_flags, int mode,
+static __device__ int warp_pack_block(const uint32_t v[4], int n, int flag, uint32_t type_flags, int mode,
                                uint64_t base64, uint8_t* sm, int dst, uint32_t* hb, int lane) {
   bool valid[4];
   uint32_t w[4];
@@ -386,7 +386,7 @@ __device__ int warp_pack_block(const uint32_t v[4], int n, int flag, uint32_t ty
 // !NoFOR && min>0 && max-min<2^32, else one block when every value fits in
 // 32 bits, else a lower-halves block (combine) followed by an upper-halves
 // block.  Returns the total length.
-__device__ int warp_pack_block64(const uint64_t x[4], int n, int flag, uint8_t* sm, int dst, uint32_t* hb, int lane) {
+static __device__ int warp_pack_block64(const uint64_t x[4], int n, int flag, uint8_t* sm, int dst, uint32_t* hb, int lane) {
   uint64_t mn = ~0ull, mx = 0ull, acc = 0ull;
 #pragma unroll
   for (int k = 0; k < 4; k++)
@@ -443,7 +443,7 @@ struct UnpackResult {
 };
 
 template <class Src>
-__device__ UnpackResult warp_unpack_block(const Src& sb, int64_t blk, int64_t avail, bool for_u64, uint32_t v[4],
+static __device__ UnpackResult warp_unpack_block(const Src& sb, int64_t blk, int64_t avail, bool for_u64, uint32_t v[4],
                                           uint32_t* hb, int lane) {
   UnpackResult r{kOK, 0, 0, 0};
   if (avail < 4) { r.status = kErrInvalidBuffer; return r; }
@@ -616,7 +616,7 @@ __device__ UnpackResult warp_unpack_block(const Src& sb, int64_t blk, int64_t av
 
 // Unpack one uint64 block (unpackUint64Block, uint64.go:191-266).
 template <class Src>
-__device__ UnpackResult warp_unpack_block64(const Src& sb, int64_t blk, int64_t avail, uint64_t out[4], uint32_t* hb,
+static __device__ UnpackResult warp_unpack_block64(const Src& sb, int64_t blk, int64_t avail, uint64_t out[4], uint32_t* hb,
                                             int lane) {
   UnpackResult r{kOK, 0, 0, 0};
   if (avail < 4) { r.status = kErrInvalidBuffer; return r; }
@@ -675,7 +675,7 @@ __device__ __forceinline__ uint32_t extract_packed(const GlobalBytes& g, int64_t
 }
 
 // svb.go:40-100: region [x, x+len) of g.
-__device__ uint32_t svb_decode_one(const GlobalBytes& g, int64_t x, int64_t len, int count, int index) {
+static __device__ uint32_t svb_decode_one(const GlobalBytes& g, int64_t x, int64_t len, int count, int index) {
   if (count <= 0 || index < 0 || index >= count) return 0;
   int64_t off = (count + 3) >> 2;
   int tcb = index >> 2, slot = index & 3;
@@ -759,7 +759,7 @@ __device__ __forceinline__ int delta_full_unpack_threshold(int bw) { return bw >
 
 // getUint32Scalar (get.go:81-190).  len is the caller's buffer length (the
 // reference's len(src)); g bounds the bytes actually readable.
-__device__ GetResult thread_get_u32(const GlobalBytes& g, int64_t len, int pos, bool for_u64) {
+static __device__ GetResult thread_get_u32(const GlobalBytes& g, int64_t len, int pos, bool for_u64) {
   GetResult r{kOK, 0, 0u, false, 0};
   if (len < 4) { r.status = kErrInvalidBuffer; return r; }
   const uint32_t h = g.u32(0);

@@ -93,7 +93,7 @@ cudaError_t plain_get(bool u64, int pos, const uint8_t* src, int64_t staged, int
                       PlainResult* res, cudaStream_t st);
 size_t index_scratch_bytes(uint64_t len);
 int index_stream(const uint8_t* p, uint64_t len, uint64_t* block_off, int64_t max_blocks, int64_t* n_blocks,
-                 void* scratch, cudaStream_t st, cudaError_t* cerr);
+                 void* scratch, void* res_d, const void* res_h, cudaStream_t st, cudaError_t* cerr);
 int set_knob(int knob, int value);
 int get_knob(int knob);
 uint32_t spin_limit();     // UTL_KNOB_SPIN_LIMIT as a poll count

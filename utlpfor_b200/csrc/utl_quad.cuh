@@ -455,7 +455,7 @@ __device__ __forceinline__ uint64_t quad_exc_from_buckets(uint32_t E, uint32_t O
 // aligned) receives the high bits in rank order and idx (16 bytes) the
 // position list or bitmap.  mode as in warp_pack_block.  Partial blocks
 // (n < 128) take masked variants of the steps that must skip padding.
-__device__ QPlan quad_plan_block(uint32_t (&x)[8][4], int n, int flag, uint32_t type_flags, int mode,
+static __device__ QPlan quad_plan_block(uint32_t (&x)[8][4], int n, int flag, uint32_t type_flags, int mode,
                                  uint32_t* hb, uint8_t* idx, uint32_t* xs, int j, unsigned qm) {
   const bool full = n == kBlock;
 #define QVALID(v, k) (16 * (v) + 4 * j + (k) < n)
@@ -628,7 +628,7 @@ __device__ QPlan quad_plan_block(uint32_t (&x)[8][4], int n, int flag, uint32_t 
 // Phase C: write the block's bytes at o (shared or global memory).  x holds
 // the work values of phase A, hb/idx its exception data.  base64 is the
 // FOR64 base.
-__device__ void quad_write_block(const QPlan& p, const uint32_t (&x)[8][4], int mode, uint64_t base64,
+static __device__ void quad_write_block(const QPlan& p, const uint32_t (&x)[8][4], int mode, uint64_t base64,
                                  const uint32_t* hb, const uint8_t* idx, uint8_t* o, int j, unsigned qm) {
   const int bw = p.bw;
   if (j == 0) {
