@@ -10,9 +10,9 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libutlpfor_b200.so")
-SOURCES = ["utl_kernels.cu", "utl_capi.cu", "utl_noalloc.cu", "utl_index.cu"]
+SOURCES = ["utl_kernels.cu", "utl_get.cu", "utl_capi.cu", "utl_noalloc.cu", "utl_index.cu"]
 HEADERS = ["utl_device.cuh", "utl_launch.h", "utl_quad.cuh", "utl_lane.cuh", "utl_pieces.h", "utl_unpack.cuh", "utl_pair.cuh",
-           "utl_unlane.cuh"]
+           "utl_unlane.cuh", "utl_get.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -35,7 +35,7 @@ def _stale():
 def build(force=False, verbose=False):
     if not force and not _stale():
         return LIB
-    cmd = [nvcc_path(), *ARCH, "-lineinfo", "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
+    cmd = [nvcc_path(), *ARCH, "-lineinfo", "-O3", "-std=c++17", "--threads", "0", "-shared", "-Xcompiler", "-fPIC",
            "-Xcompiler", "-fvisibility=hidden", "-o", LIB + ".tmp"]
     cmd += [os.path.join(CSRC, f) for f in SOURCES]
     if verbose:

@@ -25,6 +25,7 @@
 #include "utl_unpack.cuh"
 #include "utl_pair.cuh"
 #include "utl_unlane.cuh"
+#include "utl_get.cuh"
 
 namespace utl {
 
@@ -2561,143 +2562,6 @@ __global__ void __launch_bounds__(32, SHAPE == 1 ? 18 : 16) pack_pair_kernel(Pac
 }
 
 // ------------------------------------------------------------------------
-// Get: one thread per query; queries that need the reference's full-block
-// fallback (delta blocks, deep positions) are resolved by the whole warp.
-// ------------------------------------------------------------------------
-struct SubGet {
-  const uint8_t* p;  // sub-block start
-  int64_t rd;        // readable bytes
-  int64_t len;       // the reference's len(src)
-  int pos;
-};
-
-// Resolve every lane whose r.need_full is set with a warp-wide unpack of
-// its block (getUint32FullUnpack / getFullUnpackViaBlock, get.go:198-218,
-// 339-349), bounded by the block end the thread validated.
-template <bool U64>
-__device__ __forceinline__ void resolve_full(bool active, const SubGet& q, GetResult& r, uint32_t* hb, int lane) {
-  unsigned m = __ballot_sync(kFull, active && r.need_full);
-  while (m) {
-    const int src = __ffs(m) - 1;
-    m &= m - 1;
-    const uint8_t* p = (const uint8_t*)__shfl_sync(kFull, (unsigned long long)q.p, src);
-    const int64_t rd = (int64_t)__shfl_sync(kFull, (unsigned long long)q.rd, src);
-    const int64_t len = (int64_t)__shfl_sync(kFull, (unsigned long long)r.end, src);
-    const int pos = __shfl_sync(kFull, q.pos, src);
-    uint32_t v[4];
-    const GlobalBytes g{p, rd};
-    const UnpackResult u = warp_unpack_block(g, 0, len, U64, v, hb, lane);
-    const int slot = pos >> 5;
-    uint32_t mine = slot == 0 ? v[0] : slot == 1 ? v[1] : slot == 2 ? v[2] : v[3];
-    const uint32_t val = __shfl_sync(kFull, mine, pos & 31);
-    if (lane == src) {
-      r.need_full = false;
-      r.status = u.status;
-      r.ovf = u.ovf;
-      r.value = val;
-    }
-  }
-}
-
-template <bool U64>
-__global__ void __launch_bounds__(kThreads) get_kernel(GetArgs a) {
-  __shared__ uint32_t hb_all[kWarps * kBlock];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t* hb = hb_all + warp * kBlock;
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool act = q < a.n_queries;
-
-  int status = kOK, ovf = 0;
-  uint64_t result = 0;
-  SubGet sg{nullptr, 0, 0, 0};
-  bool live = false;
-  if (act) {
-    const uint32_t s = a.q_stream[q];
-    const uint64_t p = a.q_pos[q];
-    if (s >= (uint32_t)a.n_streams || p >= a.val_off[s + 1] - a.val_off[s]) {
-      status = kErrPositionOutOfRange;
-    } else {
-      const int64_t b = (int64_t)a.block_start[s] + (int64_t)(p / kBlock);
-      const uint64_t off = a.block_off[b], end = a.block_off[b + 1];
-      const uint64_t e2 = min(end, a.packed_len);
-      const int64_t rd = (e2 > off) ? (int64_t)(e2 - off) : 0;
-      sg = SubGet{a.packed + off, rd, (end >= off) ? (int64_t)(end - off) : 0, (int)(p % kBlock)};
-      live = true;
-    }
-  }
-
-  if (!U64) {
-    GetResult r{kOK, 0, 0u, false};
-    if (live) r = thread_get_u32(GlobalBytes{sg.p, sg.rd}, sg.len, sg.pos, false);
-    resolve_full<false>(live, sg, r, hb, lane);
-    if (live) {
-      status = r.status;
-      ovf = r.ovf;
-      result = r.value;
-    }
-  } else {
-    // getUint64Scalar, uint64.go:372-436
-    const GlobalBytes g{sg.p, sg.rd};
-    uint32_t h = 0;
-    bool go = live;
-    if (go) {
-      if (sg.len < 4) { status = kErrInvalidBuffer; go = false; }
-      else {
-        h = g.u32(0);
-        if (((h >> 13) & 3) != 3) { status = kErrUnsupportedType; go = false; }
-      }
-    }
-    GetResult r{kOK, 0, 0u, false};
-    if (go) r = thread_get_u32(g, sg.len, sg.pos, true);
-    resolve_full<true>(go, sg, r, hb, lane);
-    if (go && r.status != kOK) { status = r.status; ovf = r.ovf; go = false; }
-    const uint32_t lower = r.value;
-    const int forw = (int)((h >> 15) & 3), exc = (int)(h >> 24);
-    SubGet sg2{nullptr, 0, 0, sg.pos};
-    bool second = false;
-    if (go) {
-      if (!(h & kHdrCombine)) {
-        uint64_t base = 0;
-        if (forw == 3) {
-          const int off = 4 + (exc > 0 ? 2 : 0);
-          if (sg.len < off + 8) { status = kErrInvalidBuffer; go = false; }
-          else base = g.u64(off);
-        }
-        if (go) result = (uint64_t)lower + base;
-      } else {
-        const int64_t meta = 4 + (exc > 0 ? 2 : 0) + ((1 << forw) >> 1) + 2;
-        if (sg.len < meta) { status = kErrInvalidBuffer; go = false; }
-        else {
-          const int64_t b2len = g.u16(meta - 2);
-          int64_t b1 = meta + (int64_t)(((h >> 8) & 31) * 4) * 16;
-          if (exc > 0) b1 += min(exc, 16) + (int64_t)g.u16(4);
-          if (b1 + b2len > sg.len) { status = kErrInvalidBuffer; go = false; }
-          else {
-            const int64_t rd2 = max((int64_t)0, min(b2len, sg.rd - b1));
-            sg2 = SubGet{sg.p + b1, rd2, b2len, sg.pos};
-            second = true;
-          }
-        }
-      }
-    }
-    GetResult r2{kOK, 0, 0u, false};
-    if (second) r2 = thread_get_u32(GlobalBytes{sg2.p, sg2.rd}, sg2.len, sg2.pos, true);
-    resolve_full<true>(second, sg2, r2, hb, lane);
-    if (second) {
-      if (r2.status != kOK) { status = r2.status; ovf = r2.ovf; }
-      else result = ((uint64_t)r2.value << 32) | lower;
-    }
-  }
-
-  if (act) {
-    if (U64) ((uint64_t*)a.out)[q] = status == kOK ? result : 0ull;
-    else ((uint32_t*)a.out)[q] = status == kOK ? (uint32_t)result : 0u;
-    if (a.status) a.status[q] = status | (ovf << 8);
-    if (status != kOK && a.err) atomicOr(a.err, 1u << status);
-  }
-}
-
-// ------------------------------------------------------------------------
 // per-call kernels (one warp): inputs and outputs live in mapped pinned
 // host memory, so a call is one launch and one synchronize.
 // ------------------------------------------------------------------------
@@ -3256,15 +3120,6 @@ cudaError_t unpack(bool u64, const UnpackArgs& a, cudaStream_t st) {
   }
   const int64_t grid = tiles_for(a.n_blocks);
   unpack_kernel<true><<<(unsigned)grid, kThreads, unpack_smem(true), st>>>(a);
-  note_launch(1);
-  return cudaGetLastError();
-}
-
-cudaError_t get(bool u64, const GetArgs& a, cudaStream_t st) {
-  if (a.n_queries <= 0) return cudaSuccess;
-  const int64_t grid = (a.n_queries + kThreads - 1) / kThreads;
-  if (u64) get_kernel<true><<<(unsigned)grid, kThreads, 0, st>>>(a);
-  else get_kernel<false><<<(unsigned)grid, kThreads, 0, st>>>(a);
   note_launch(1);
   return cudaGetLastError();
 }
