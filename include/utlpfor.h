@@ -321,10 +321,13 @@ UTL_API int utl_index_stream(const uint8_t *d_packed, size_t packed_len,
  *     bytes a block on average, else 2, decided on the device (the default).
  *   UTL_KNOB_PACK_CTAS_PER_SM: cap on resident pack CTAs per SM (0 = the
  *     occupancy maximum).
- *   UTL_KNOB_PACK_SCHEDULE: uint32 pack kernel, 0 = four threads per block
- *     (CTA tiles), 1 = one thread per block (independent warp tiles of 32
- *     blocks), 2 = a lane pair per block (independent warp tiles of 16
- *     blocks, half the shared memory per warp, more warps per SM).
+ *   UTL_KNOB_PACK_SCHEDULE: the pack kernel, 0 = four threads per block
+ *     (CTA tiles; uint64: a warp per block), 1 = one thread per block
+ *     (independent warp tiles of 32 blocks), 2 = a lane pair per block
+ *     (uint32; independent warp tiles of 16 blocks, half the shared memory per
+ *     warp, more warps per SM), 3 = two launches of four lanes per block
+ *     (plans, then bytes) for uint64, NoPatch and small batches, 1 for the
+ *     others (the default).
  *   UTL_KNOB_PACK_WINDOW: the tile image of the one-thread and lane-pair
  *     packs, 0 = by the block density of the previous pack on this device
  *     that may allocate (a hint read without waiting), 1 = the large window,

@@ -10,9 +10,10 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libutlpfor_b200.so")
-SOURCES = ["utl_kernels.cu", "utl_get.cu", "utl_capi.cu", "utl_noalloc.cu", "utl_index.cu"]
+SOURCES = ["utl_kernels.cu", "utl_pack.cu", "utl_get.cu", "utl_capi.cu", "utl_noalloc.cu", "utl_index.cu"]
 HEADERS = ["utl_device.cuh", "utl_launch.h", "utl_quad.cuh", "utl_lane.cuh", "utl_pieces.h", "utl_unpack.cuh", "utl_pair.cuh",
-           "utl_unlane.cuh", "utl_get.cuh"]
+           "utl_unlane.cuh", "utl_get.cuh",
+           "utl_qpack.cuh", "utl_streams.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -581,7 +581,8 @@ int utl::pack_batch_device(bool u64, bool may_alloc, uint8_t flag, const void* d
     UTL_CUDA(cudaMemsetAsync(d_block_off, 0, sizeof(uint64_t), st));
   } else {
     if (scratch_bytes < launch::pack_scratch_bytes(n_blocks)) return UTL_ERR_ARG;
-    if (!launch::keep_scratch()) UTL_CUDA(cudaMemsetAsync(d_scratch, 0, launch::pack_scratch_bytes(n_blocks), st));
+    if (launch::pack_needs_clear(u64, flag, n_blocks))
+      UTL_CUDA(cudaMemsetAsync(d_scratch, 0, launch::pack_scratch_bytes(n_blocks), st));
     PackArgs a;
     a.values = d_values;
     a.val_off = d_val_off;

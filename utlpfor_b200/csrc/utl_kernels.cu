@@ -20,6 +20,7 @@
 
 #include "utl_device.cuh"
 #include "utl_launch.h"
+#include "utl_streams.cuh"
 #include "utl_lane.cuh"
 #include "utl_quad.cuh"
 #include "utl_unpack.cuh"
@@ -87,45 +88,6 @@ __device__ __forceinline__ void block_span(const uint64_t* val_off, const uint64
   *n = (int)min((uint64_t)kBlock, e - f);
 }
 
-// Stream of block b (largest s with block_start[s] <= b).
-__device__ __forceinline__ int stream_of(const uint64_t* bstart, int n_streams, int64_t b) {
-  int lo = 0, hi = n_streams;
-  while (hi - lo > 1) {
-    int mid = (lo + hi) >> 1;
-    if ((int64_t)bstart[mid] <= b) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-// The same by the whole warp, each round probing 32 evenly spaced streams at
-// once: two dependent loads for 1000 streams where the bisection takes ten.
-__device__ __forceinline__ int warp_stream_of(const uint64_t* bstart, int n_streams, int64_t b, int lane) {
-  int lo = 0, hi = n_streams;
-  while (hi - lo > 1) {
-    const int step = (hi - lo + 31) >> 5;
-    const int64_t p = (int64_t)lo + (int64_t)lane * step;
-    const unsigned m = __ballot_sync(kFull, p < hi && (lane == 0 || (int64_t)bstart[p] <= b));
-    lo += (31 - __clz(m)) * step;
-    hi = min(hi, lo + step);
-  }
-  return lo;
-}
-// The same, knowing the stream s0 of an earlier block: galloping from s0
-// (consecutive blocks are nearly always in the same or the next stream).
-__device__ __forceinline__ int stream_from(const uint64_t* bstart, int n_streams, int s0, int64_t b) {
-  int lo = s0, step = 1;
-  while (lo + step < n_streams && (int64_t)bstart[lo + step] <= b) {
-    lo += step;
-    step <<= 1;
-  }
-  int hi = min(n_streams, lo + step);
-  while (hi - lo > 1) {
-    int mid = (lo + hi) >> 1;
-    if ((int64_t)bstart[mid] <= b) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
 // First value index and value count of block b of stream s.
 __device__ __forceinline__ void span_in(const uint64_t* val_off, const uint64_t* bstart, int s, int64_t b,
                                         uint64_t* first, int* n) {
@@ -2902,7 +2864,7 @@ static cudaError_t unpack_tma(const UnpackArgs& a, cudaStream_t st, int ctas) {
 // UTL_KNOB_UNPACK_SCHEDULE (include/utlpfor.h)
 static int g_unpack_schedule = 8;
 static int g_pack_cap = 0;
-static int g_pack_schedule = 1;
+static int g_pack_schedule = 3;
 // Test knobs: the polls of every bounded wait (0 = the default 2^22), and
 // whether the pack leaves the caller's scratch as it finds it.
 static std::atomic<uint32_t> g_spin_limit{0};
@@ -3051,10 +3013,16 @@ static cudaError_t pack_lane(const PackArgs& a_in, cudaStream_t st, bool u64, bo
   return cudaGetLastError();
 }
 
+bool pack_needs_clear(bool u64, int flag, int64_t n_blocks) {
+  if (g_keep_scratch.load(std::memory_order_relaxed)) return false;
+  return !(g_pack_schedule == 3 && pack_by_two(u64, flag, n_blocks)) || pack_two_clears(n_blocks);
+}
+
 cudaError_t pack(bool u64, const PackArgs& a_in, cudaStream_t st, bool may_alloc) {
   DevCfg* c = nullptr;
   cudaError_t e = dev_cfg(&c);
   if (e != cudaSuccess) return e;
+  if (g_pack_schedule == 3 && pack_by_two(u64, a_in.flag, a_in.n_blocks)) return pack_two(u64, a_in, st);
   if (g_pack_schedule == 2 && !u64) return pack_pair(a_in, st, may_alloc, *c);
   if (g_pack_schedule >= 1) return pack_lane(a_in, st, u64, may_alloc, *c);
   if (!u64) {
@@ -3171,7 +3139,7 @@ int set_knob(int knob, int value) {
       g_pack_cap = value;
       return 0;
     case 2:  // UTL_KNOB_PACK_SCHEDULE
-      if (value < 0 || value > 2) return -1;
+      if (value < 0 || value > 3) return -1;
       g_pack_schedule = value;
       return 0;
     case 7:  // UTL_KNOB_UNPACK_CTAS_PER_SM (0 = occupancy maximum)

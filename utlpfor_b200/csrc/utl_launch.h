@@ -84,6 +84,12 @@ cudaError_t stream_offsets(const uint64_t* block_off, const uint64_t* bstart, in
 // may_alloc false: the launch makes no allocation of any kind (the uint32
 // lane pack then skips its mapped-memory window hint).
 cudaError_t pack(bool u64, const PackArgs& a, cudaStream_t st, bool may_alloc);
+// utl_pack.cu: the pack in two launches, the batches that take it by default,
+// and whether it needs its scratch cleared.
+cudaError_t pack_two(bool u64, const PackArgs& a, cudaStream_t st);
+bool pack_by_two(bool u64, int flag, int64_t n_blocks);
+bool pack_two_clears(int64_t n_blocks);
+bool pack_needs_clear(bool u64, int flag, int64_t n_blocks);  // of the schedule in force
 cudaError_t unpack(bool u64, const UnpackArgs& a, cudaStream_t st);
 cudaError_t get(bool u64, const GetArgs& a, cudaStream_t st);
 cudaError_t plain_pack(bool u64, int flag, const void* vals, int n, uint8_t* out, PlainResult* res, cudaStream_t st);

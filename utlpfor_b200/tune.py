@@ -7,7 +7,8 @@ that file (if any) for the current GPU and sets the knobs.  Knobs
 (include/utlpfor.h):
   2 UTL_KNOB_PACK_SCHEDULE       blocks per warp tile: 2 = 16 (lane pair per
                                  block), 1 = 32 (one thread per block),
-                                 0 = four threads per block, CTA tiles
+                                 0 = four threads per block, CTA tiles;
+                                 3 = two launches or 1, by the batch
   6 UTL_KNOB_PACK_WINDOW         1 large / 2 small tile image (warps per SM)
   1 UTL_KNOB_PACK_CTAS_PER_SM    0 occupancy maximum, else a cap
   0 UTL_KNOB_UNPACK_SCHEDULE     0 tiles; 1-3 cp.async double buffer (auto,
@@ -37,7 +38,7 @@ TUNED = os.path.join(HERE, "tuned")
 # unpack staging size stay chosen per batch (window 0, unpack schedules 1,
 # 4 and 8 pick by block density), so a setting tuned on one workload cannot
 # slow down a batch of much larger blocks.
-PACK_SHAPES = [(1, 0), (2, 0), (0, 0)]  # (schedule, window)
+PACK_SHAPES = [(3, 0), (2, 0), (0, 0)]  # (schedule, window); 3 is 1 on the swept batch
 PACK_CAPS = [0, 16, 12, 8]
 UNPACK_SCHEDULES = [8, 1, 4, 0]
 UNPACK_CAPS = [0, 4, 3, 2]
