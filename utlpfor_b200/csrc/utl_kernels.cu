@@ -1170,17 +1170,23 @@ __global__ void __launch_bounds__(32 * W, 16 / W) unpack_lane_kernel(UnpackArgs 
 }
 
 // The default uint32 unpack in one launch: the thread-per-block path for
-// batches of at most kWideMean bytes a block on average, the quad pipeline
-// with the large staging otherwise (both persistent, 4 warps per CTA, at
+// large batches of at most kWideMean bytes a block on average, the quad
+// pipeline with the large staging otherwise (both persistent, 4 warps per CTA, at
 // most as much shared memory as the launch provides), chosen from the
 // block offsets by every CTA alike.
 constexpr size_t kAutoSmem = sizeof(LaneUnpackSmem<1, kLUStage1, 4>) > sizeof(QuadPipeSmem<kPStageWide, 2>)
                                  ? sizeof(LaneUnpackSmem<1, kLUStage1, 4>)
                                  : sizeof(QuadPipeSmem<kPStageWide, 2>);
+// Up to two groups of eight blocks for every resident warp the quad pipeline
+// is taken whatever the mean length: a warp's 32 blocks one after the other
+// leave most of the SMs idle.  2^20 postings in 128 lists 28.7 -> 12.3 us, 2^22
+// 28.7 -> 22.6, 2^22 outlier values 12.3 -> 10.3; at 2^23 it is the slower one
+// (outliers 14.3 -> 16.4).
+constexpr int64_t kQuadBlocks = 148 * 16 * 8 * 2;
 __global__ void __launch_bounds__(kQThreads, 4) unpack_auto_kernel(UnpackArgs a) {
   extern __shared__ uint4 smem4[];
   const uint64_t span = a.block_off[a.n_blocks] - a.block_off[0];
-  if (span <= kWideMean * (uint64_t)a.n_blocks) lane_body<1, kLUStage1, 4>(a, smem4);
+  if (a.n_blocks > kQuadBlocks && span <= kWideMean * (uint64_t)a.n_blocks) lane_body<1, kLUStage1, 4>(a, smem4);
   else pipe_body<kPStageWide, false, 2>(a, smem4);
 }
 
