@@ -50,6 +50,7 @@ static inline uint32_t ld32(const uint8_t* p) {
 constexpr size_t kStageIn = 144 * 1024;  // covers the largest span a corrupt block can name
 constexpr size_t kStageOut = 4096;       // one packed block (<= 2038 B) or 128 values
 constexpr size_t kStageRes = 256;
+static_assert(kStageIn % 16 == 0, "staged input is read in whole 16-byte pieces");
 constexpr size_t kStageBytes = kStageIn + kStageOut + kStageRes;
 
 struct Grow {
