@@ -651,8 +651,12 @@ def main():
     dom_achieved = pack_gbs if dom == "pack" else unpack_gbs
     pack_names = {0: "pack_quad_kernel", 1: "pack_lane_kernel", 2: "pack_pair_kernel"}
     if dom == "pack":
-        kname = ("pack_kernel" if L.utl_get_knob(2) == 0 else "pack_lane_kernel") if is64 else \
-            pack_names.get(L.utl_get_knob(2), "pack_lane_kernel")
+        sched = L.utl_get_knob(2)
+        # schedule 3: two launches (plan_kernel, write_kernel) for uint64, NoPatch and small batches
+        two = sched == 3 and (is64 or (flag & NOPATCH) != 0 or codec.n_blocks <= 16384)
+        kname = "plan_kernel+write_kernel" if two else \
+            ("pack_kernel" if sched == 0 else "pack_lane_kernel") if is64 else \
+            pack_names.get(sched, "pack_lane_kernel")
     elif is64:
         s64 = L.utl_get_knob(8)
         kname = "unpack_kernel" if s64 == 0 else "unpack_oct64_tma_kernel" if s64 in (1, 2) else "unpack_quad_pipe_kernel"
