@@ -323,6 +323,7 @@ constexpr int kBitWords = kSub / 32 + 1;  // their block starts as bits
 constexpr int kRegion = kSub * kTeams;    // bytes of a CTA (32 KB: six CTAs, 24 warps, on an SM)
 constexpr int kAhead = 32;                // staged bytes past the region (headers that start in it)
 static_assert(kRegion % 16 == 0, "regions keep the stream's alignment");
+constexpr uint32_t kDrainPolls = 1u << 22;  // for a copy that must land before the CTA ends, whatever the knob says
 
 // Result of the first path: the block count, and whether it holds.
 struct FastResult {
@@ -461,9 +462,18 @@ __global__ void __launch_bounds__(kRT) index_starts_kernel(const uint8_t* p, uin
   for (uintptr_t a = a0 + k; a < e0; a += kRT) ((uint8_t*)buf)[a - a0] = a >= lo && a < hi ? *(const uint8_t*)a : 0;
   if (bulk)
     for (uintptr_t a = t1 + k; a < a1; a += kRT) ((uint8_t*)buf)[a - a0] = a < hi ? *(const uint8_t*)a : 0;
+  if (__syncthreads_or(bulk && !tma::mbar_wait(&bar, 0, spin))) {
+    // The copy did not land within the limit: nothing in buf is looked at.
+    // The call is left to the second path, and the copy gets the full limit
+    // to land before the CTA's shared memory goes to another one.
+    if (k == 0) {
+      *(volatile int64_t*)&tab.exits[r] = -1;
+      atomicOr(&tab.ctl->bad, 1u);
+    }
+    tma::mbar_wait(&bar, 0, kDrainPolls);
+    return;
+  }
   bool failed = false;
-  if (bulk) failed = !tma::mbar_wait(&bar, 0, spin);
-  __syncthreads();
 
   // a start per team, guessed: the four threads look at alternate pairs of words
   const int team = k / kTeam, c4 = k % kTeam;
