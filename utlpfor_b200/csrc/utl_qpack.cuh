@@ -346,27 +346,37 @@ __device__ __forceinline__ void put_exceptions(const uint32_t (&x)[8][4], const 
   const bool list = exc <= 16;
   const int nc = (exc + 3) >> 2;
   uint8_t* svb = xi + min(exc, 16);
-  uint32_t ctrl = 0;
-  int tot = 0, rank = first;
-  for (uint32_t b = W; b; b &= b - 1, rank++) {
-    const int pos = 32 * j + __ffs(b) - 1;
-    const int code = (31 - __clz(slot[pos] >> bw)) >> 3;  // StreamVByte length - 1
-    if (list) xi[rank] = (uint8_t)pos;
-    ctrl |= quad::shl_clamp((uint32_t)code, 2u * (uint32_t)rank);
-    tot += code + 1;
-  }
   if (!list) {
     put4(xi + 4 * j, W, 4);
     for (int g = j; g < nc; g += 4) svb[g] = 0;
   }
   __syncwarp();
+  // The codes.  With more than 16 exceptions the lanes share control bytes and
+  // OR their codes into the aligned word.  That word may reach into the bitmap
+  // before and the data after (never out of the block's own bytes: there are 16
+  // bytes of bitmap and at least 17 of data), so both are written on the other
+  // side of a barrier: an atomic leaves no order between itself and a plain
+  // store to its word.
+  uint32_t ctrl = 0;
+  int tot = 0, rank = first;
+  for (uint32_t b = W; b; b &= b - 1, rank++) {
+    const int pos = 32 * j + __ffs(b) - 1;
+    const int code = (31 - __clz(slot[pos] >> bw)) >> 3;  // StreamVByte length - 1
+    if (list) {
+      xi[rank] = (uint8_t)pos;
+      ctrl |= (uint32_t)code << (2 * rank);
+    } else if (code) {
+      const uintptr_t g = (uintptr_t)(svb + (rank >> 2));
+      atomicOr((uint32_t*)(g & ~(uintptr_t)3), (uint32_t)code << (8 * (int)(g & 3) + 2 * (rank & 3)));
+    }
+    tot += code + 1;
+  }
   int d = nc + (int)q_excl((uint32_t)tot, j);
   ctrl = q_or(ctrl);
   if (list && j < nc) svb[j] = (uint8_t)(ctrl >> (8 * j));
-  rank = first;
-  for (uint32_t b = W; b; b &= b - 1, rank++) {
-    const int pos = 32 * j + __ffs(b) - 1;
-    const uint32_t hv = slot[pos] >> bw;
+  __syncwarp();
+  for (uint32_t b = W; b; b &= b - 1) {
+    const uint32_t hv = slot[32 * j + __ffs(b) - 1] >> bw;
     const int code = (31 - __clz(hv)) >> 3;
     uint8_t* p = svb + d;
     p[0] = (uint8_t)hv;
@@ -374,11 +384,6 @@ __device__ __forceinline__ void put_exceptions(const uint32_t (&x)[8][4], const 
     if (code > 1) p[2] = (uint8_t)(hv >> 16);
     if (code > 2) p[3] = (uint8_t)(hv >> 24);
     d += code + 1;
-    if (!list && code) {
-      // lanes share control bytes: OR the code into its aligned word
-      const uintptr_t g = (uintptr_t)(svb + (rank >> 2));
-      atomicOr((uint32_t*)(g & ~(uintptr_t)3), (uint32_t)code << (8 * (int)(g & 3) + 2 * (rank & 3)));
-    }
   }
 }
 
