@@ -2779,13 +2779,21 @@ static cudaError_t dev_cfg(DevCfg** out) {
   return cudaSuccess;
 }
 
-// The mapped pinned stats pair of a device (allocating; once per device).
+// The mapped pinned stats pair of a device (allocating; once per device, by
+// the first pack that may allocate, whichever kernels it takes).  A first use
+// may fall into a stream capture, of this thread or another: an allocation
+// orders nothing that is captured, so the thread allows itself the call, which
+// would otherwise end the capture.
 static uint64_t* lane_stats_dev(DevCfg& c) {
   if (c.stats.load(std::memory_order_acquire)) return c.stats_dev;
   std::lock_guard<std::mutex> lk(g_setup_mu);
   if (c.stats.load(std::memory_order_relaxed)) return c.stats_dev;
   uint64_t* h = nullptr;
-  if (cudaHostAlloc((void**)&h, 2 * sizeof(uint64_t), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+  const cudaError_t got = cudaHostAlloc((void**)&h, 2 * sizeof(uint64_t), cudaHostAllocMapped | cudaHostAllocPortable);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (got != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
@@ -2976,7 +2984,7 @@ static cudaError_t setup_device(int dev, DevCfg& c) {
   c.pipe64_ctas[2] = occupancy(unpack_quad_pipe_kernel<kP64StageWide, false, true, 1>, kQThreads, q1);
   if ((e = set_smem(unpack_kernel<false>, unpack_smem(false))) != cudaSuccess) return e;
   if ((e = set_smem(unpack_kernel<true>, unpack_smem(true))) != cudaSuccess) return e;
-  return cudaSuccess;
+  return pack_two_setup();
 }
 
 // Window shape of a uint32 pack (0 large, 1 small): the knob, or the block
@@ -3045,6 +3053,7 @@ cudaError_t pack(bool u64, const PackArgs& a_in, cudaStream_t st, bool may_alloc
   DevCfg* c = nullptr;
   cudaError_t e = dev_cfg(&c);
   if (e != cudaSuccess) return e;
+  if (may_alloc) lane_stats_dev(*c);
   if (g_pack_schedule == 3 && pack_by_two(u64, a_in.flag, a_in.n_blocks)) return pack_two(u64, a_in, st);
   if (g_pack_schedule == 2 && !u64) return pack_pair(a_in, st, may_alloc, *c);
   if (g_pack_schedule >= 1) return pack_lane(a_in, st, u64, may_alloc, *c);

@@ -84,8 +84,10 @@ cudaError_t stream_offsets(const uint64_t* block_off, const uint64_t* bstart, in
 // may_alloc false: the launch makes no allocation of any kind (the uint32
 // lane pack then skips its mapped-memory window hint).
 cudaError_t pack(bool u64, const PackArgs& a, cudaStream_t st, bool may_alloc);
-// utl_pack.cu: the pack in two launches, the batches that take it by default,
+// utl_pack.cu: the pack in two launches, its kernels' attributes (set with the
+// other kernels' on a device's first use), the batches that take it by default,
 // and whether it needs its scratch cleared.
+cudaError_t pack_two_setup();
 cudaError_t pack_two(bool u64, const PackArgs& a, cudaStream_t st);
 bool pack_by_two(bool u64, int flag, int64_t n_blocks);
 bool pack_two_clears(int64_t n_blocks);

@@ -19,9 +19,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <atomic>
-#include <mutex>
-
 #include "utl_launch.h"
 #include "utl_qpack.cuh"
 #include "utl_streams.cuh"
@@ -360,23 +357,12 @@ static cudaError_t pack_attr() {
   if (e == cudaSuccess) cudaFuncSetAttribute((const void*)k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   return e;
 }
-// Kernel attributes, set once per device under a lock with it current.
-static cudaError_t pack_setup() {
-  static std::atomic<int> ready[64];
-  static std::mutex mu;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (ready[dev].load(std::memory_order_acquire)) return cudaSuccess;
-  std::lock_guard<std::mutex> lk(mu);
-  if (ready[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+cudaError_t pack_two_setup() {
+  cudaError_t e;
   if ((e = pack_attr<false, false>()) != cudaSuccess) return e;
   if ((e = pack_attr<true, false>()) != cudaSuccess) return e;
   if ((e = pack_attr<false, true>()) != cudaSuccess) return e;
-  if ((e = pack_attr<true, true>()) != cudaSuccess) return e;
-  ready[dev].store(1, std::memory_order_release);
-  return cudaSuccess;
+  return pack_attr<true, true>();
 }
 
 template <bool DELTA, bool U64>
@@ -410,8 +396,7 @@ bool pack_by_two(bool u64, int flag, int64_t n_blocks) {
 bool pack_two_clears(int64_t n_blocks) { return n_blocks > (int64_t)qp::kDirectTiles * qp::kTile; }
 
 cudaError_t pack_two(bool u64, const PackArgs& a_in, cudaStream_t st) {
-  cudaError_t e = pack_setup();
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   PackArgs a = a_in;
   a.n_tiles = (a.n_blocks + qp::kTile - 1) / qp::kTile;
   if (a.n_tiles > INT32_MAX) return cudaErrorInvalidValue;
