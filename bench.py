@@ -652,8 +652,11 @@ def main():
     pack_names = {0: "pack_quad_kernel", 1: "pack_lane_kernel", 2: "pack_pair_kernel"}
     if dom == "pack":
         sched = L.utl_get_knob(2)
-        # schedule 3: two launches (plan_kernel, write_kernel) for uint64, NoPatch and small batches
-        two = sched == 3 and (is64 or (flag & NOPATCH) != 0 or codec.n_blocks <= 16384)
+        # schedule 3 takes one launch or two by the batch: counted on one more pack
+        launches0 = L.utl_launch_count()
+        codec.pack(values)
+        torch.cuda.synchronize()
+        two = L.utl_launch_count() - launches0 == 2
         kname = "plan_kernel+write_kernel" if two else \
             ("pack_kernel" if sched == 0 else "pack_lane_kernel") if is64 else \
             pack_names.get(sched, "pack_lane_kernel")

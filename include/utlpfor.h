@@ -326,11 +326,13 @@ UTL_API int utl_index_stream(const uint8_t *d_packed, size_t packed_len,
  *     (independent warp tiles of 32 blocks), 2 = a lane pair per block
  *     (uint32; independent warp tiles of 16 blocks, half the shared memory per
  *     warp, more warps per SM), 3 = two launches of four lanes per block
- *     (plans, then bytes) for uint64, NoPatch and small batches, 1 for the
- *     others (the default).
+ *     (plans, then bytes) for uint64 and small batches and for large NoPatch
+ *     ones while the last of those on this device averaged more than 224 bytes
+ *     a block (a hint as below), 1 for the others (the default).
  *   UTL_KNOB_PACK_WINDOW: the tile image of the one-thread and lane-pair
- *     packs, 0 = by the block density of the previous pack on this device
- *     that may allocate (a hint read without waiting), 1 = the large window,
+ *     packs, 0 = by the block density of the previous such pack on this
+ *     device, with or without NoPatch as this one, that may allocate (a hint
+ *     read without waiting), 1 = the large window,
  *     2 = the small window (for batches of at most about 144 bytes a block).
  *     Outputs are the same for every value.
  *   UTL_KNOB_UNPACK_CTAS_PER_SM: cap on resident CTAs (4 warps each) per SM

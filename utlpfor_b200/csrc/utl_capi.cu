@@ -582,7 +582,10 @@ int utl::pack_batch_device(bool u64, bool may_alloc, uint8_t flag, const void* d
     UTL_CUDA(cudaMemsetAsync(d_block_off, 0, sizeof(uint64_t), st));
   } else {
     if (scratch_bytes < launch::pack_scratch_bytes(n_blocks)) return UTL_ERR_ARG;
-    if (launch::pack_needs_clear(u64, flag, n_blocks))
+    bool two = false;
+    cudaError_t e = launch::pack_route(u64, flag, n_blocks, may_alloc, &two);
+    if (e != cudaSuccess) return cuda_fail(e);
+    if (launch::pack_needs_clear(two, n_blocks))
       UTL_CUDA(cudaMemsetAsync(d_scratch, 0, launch::pack_scratch_bytes(n_blocks), st));
     PackArgs a;
     a.values = d_values;
@@ -599,7 +602,7 @@ int utl::pack_batch_device(bool u64, bool may_alloc, uint8_t flag, const void* d
     a.tile_status = (uint64_t*)((uint8_t*)d_scratch + 16);
     a.err = d_err;
     a.spin_limit = launch::spin_limit();
-    cudaError_t e = launch::pack(u64, a, st, may_alloc);
+    e = launch::pack(u64, two, a, st, may_alloc);
     if (e != cudaSuccess) return cuda_fail(e);
   }
   if (d_sbo) {

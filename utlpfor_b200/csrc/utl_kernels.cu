@@ -2733,11 +2733,13 @@ struct DevCfg {
   int auto_unpack_ctas = 0;          // unpack_auto_kernel
   int pipe64_ctas[3] = {0, 0, 0};  // unpack_quad_pipe_kernel for uint64: narrow, wide, wide single buffer
   int pack_ctas[2] = {0, 0};     // pack_kernel<false/true>
-  // Mapped pinned pair the uint32 lane pack's last block fills with the
-  // batch's packed bytes and block count; the next allocating launch on
-  // this device reads it (without waiting) to pick its window shape.  Only
-  // a performance hint: a stale or torn pair picks the other shape, whose
-  // output is the same.  Allocated by the first pack that may allocate.
+  // Two mapped pinned pairs, for batches with and without patching: packed
+  // bytes and blocks of the device's last large uint32 batch, left there by
+  // the kernel of its last block.  The next allocating pack reads the pair of
+  // its own kind, without waiting, to pick its window shape and, under
+  // NoPatch, its kernels.  Only a performance hint: a stale or torn pair picks
+  // the other shape or kernels, whose output is the same.  Allocated by the
+  // first pack that may allocate.
   std::atomic<uint64_t*> stats{nullptr};
   uint64_t* stats_dev = nullptr;
 };
@@ -2779,7 +2781,7 @@ static cudaError_t dev_cfg(DevCfg** out) {
   return cudaSuccess;
 }
 
-// The mapped pinned stats pair of a device (allocating; once per device, by
+// The mapped pinned stats pairs of a device (allocating; once per device, by
 // the first pack that may allocate, whichever kernels it takes).  A first use
 // may fall into a stream capture, of this thread or another: an allocation
 // orders nothing that is captured, so the thread allows itself the call, which
@@ -2791,13 +2793,13 @@ static uint64_t* lane_stats_dev(DevCfg& c) {
   uint64_t* h = nullptr;
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
-  const cudaError_t got = cudaHostAlloc((void**)&h, 2 * sizeof(uint64_t), cudaHostAllocMapped | cudaHostAllocPortable);
+  const cudaError_t got = cudaHostAlloc((void**)&h, 4 * sizeof(uint64_t), cudaHostAllocMapped | cudaHostAllocPortable);
   cudaThreadExchangeStreamCaptureMode(&mode);
   if (got != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  h[0] = h[1] = 0;
+  h[0] = h[1] = h[2] = h[3] = 0;
   uint64_t* d = nullptr;
   if (cudaHostGetDevicePointer((void**)&d, h, 0) != cudaSuccess) {
     cudaGetLastError();
@@ -2987,19 +2989,32 @@ static cudaError_t setup_device(int dev, DevCfg& c) {
   return pack_two_setup();
 }
 
+// The pair of a batch's kind, and its mean block length (0: none recorded).
+static int stats_pair(int flag) { return (flag & kNoPatch) ? 2 : 0; }
+static uint64_t* stats_for(DevCfg& c, int flag, bool may_alloc) {
+  uint64_t* d = may_alloc ? lane_stats_dev(c) : nullptr;
+  return d ? d + stats_pair(flag) : nullptr;
+}
+static uint64_t stats_mean(const DevCfg& c, int pair) {
+  const volatile uint64_t* hv = c.stats.load(std::memory_order_acquire);
+  const uint64_t bytes = hv ? hv[pair] : 0, blocks = hv ? hv[pair + 1] : 0;
+  return blocks > 0 ? (bytes + blocks - 1) / blocks : 0;
+}
+
 // Window shape of a uint32 pack (0 large, 1 small): the knob, or the block
-// density of the previous allocating pack on this device, read from the
-// mapped pair without waiting (a performance hint only).  Sets a.stats for
-// the kernel to record this batch's density (allocating calls only).
+// density of the previous allocating pack of its kind on this device (of the
+// other kind, while there is none).  Sets a.stats for the kernel to record this
+// batch's density (allocating calls only).
 static int pick_window(PackArgs& a, bool may_alloc, DevCfg& c, uint64_t small_block) {
-  a.stats = may_alloc ? lane_stats_dev(c) : nullptr;
+  a.stats = stats_for(c, a.flag, may_alloc);
   const int kn = g_pack_window.load(std::memory_order_relaxed);
   if (kn == 1) return 0;
   if (kn == 2) return 1;
   if (!a.stats) return 0;
-  const volatile uint64_t* hv = c.stats.load(std::memory_order_acquire);
-  const uint64_t bytes = hv[0], blocks = hv[1];
-  return (blocks > 0 && bytes <= blocks * small_block) ? 1 : 0;
+  const int pair = stats_pair(a.flag);
+  uint64_t mean = stats_mean(c, pair);
+  if (mean == 0) mean = stats_mean(c, 2 - pair);
+  return (mean > 0 && mean <= small_block) ? 1 : 0;
 }
 
 template <bool DELTA, int SHAPE>
@@ -3044,17 +3059,31 @@ static cudaError_t pack_lane(const PackArgs& a_in, cudaStream_t st, bool u64, bo
   return cudaGetLastError();
 }
 
-bool pack_needs_clear(bool u64, int flag, int64_t n_blocks) {
-  if (g_keep_scratch.load(std::memory_order_relaxed)) return false;
-  return !(g_pack_schedule == 3 && pack_by_two(u64, flag, n_blocks)) || pack_two_clears(n_blocks);
+cudaError_t pack_route(bool u64, int flag, int64_t n_blocks, bool may_alloc, bool* two) {
+  DevCfg* c = nullptr;
+  const cudaError_t e = dev_cfg(&c);
+  if (e != cudaSuccess) return e;
+  const uint64_t mean = may_alloc && lane_stats_dev(*c) ? stats_mean(*c, stats_pair(kNoPatch)) : 0;
+  *two = g_pack_schedule == 3 && pack_by_two(u64, flag, n_blocks, mean);
+  return cudaSuccess;
 }
 
-cudaError_t pack(bool u64, const PackArgs& a_in, cudaStream_t st, bool may_alloc) {
+bool pack_needs_clear(bool two, int64_t n_blocks) {
+  if (g_keep_scratch.load(std::memory_order_relaxed)) return false;
+  return !two || pack_two_clears(n_blocks);
+}
+
+cudaError_t pack(bool u64, bool two, const PackArgs& a_in, cudaStream_t st, bool may_alloc) {
+  // uint64 and small batches, which keep their latency, leave no density
+  if (two && pack_by_two(u64, a_in.flag, a_in.n_blocks, 0)) return pack_two(u64, a_in, st);
   DevCfg* c = nullptr;
   cudaError_t e = dev_cfg(&c);
   if (e != cudaSuccess) return e;
-  if (may_alloc) lane_stats_dev(*c);
-  if (g_pack_schedule == 3 && pack_by_two(u64, a_in.flag, a_in.n_blocks)) return pack_two(u64, a_in, st);
+  if (two) {  // its route hung on the density of the batch before it
+    PackArgs a = a_in;
+    a.stats = stats_for(*c, a.flag, may_alloc);
+    return pack_two(u64, a, st);
+  }
   if (g_pack_schedule == 2 && !u64) return pack_pair(a_in, st, may_alloc, *c);
   if (g_pack_schedule >= 1) return pack_lane(a_in, st, u64, may_alloc, *c);
   if (!u64) {

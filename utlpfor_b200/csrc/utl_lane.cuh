@@ -31,8 +31,8 @@ constexpr int kMaxLen = 528;
 //   0: uint32, 7 KB (9 warps per SM);
 //   1: uint32 batches of small blocks, 4752 bytes, the largest window at
 //      which 10 warps fit an SM (227 KB of shared memory, 1 KB reserved per
-//      CTA); chosen when the previous uint32 pack averaged at most
-//      kSmallBlock bytes a block;
+//      CTA); chosen when the previous uint32 pack of this kind (with or
+//      without patching) averaged at most kSmallBlock bytes a block;
 //   2: uint64, 10 KB: its tiles run to 32 sub-blocks of up to 528 bytes.
 constexpr int kWindow = 7168;
 constexpr int kWindowSmall = 4752;
@@ -162,7 +162,7 @@ __device__ __forceinline__ uint32_t work_at(const uint32_t* s, int pos, uint32_t
 // is set so that its work values are zero, as the reference leaves them
 // (scalar.go:34-40, delta.go:23-48): base in row 0, the lane's value one
 // row up below it.
-__device__ __noinline__ void fill_padding(uint32_t* s, int n, uint32_t base) {
+static __device__ __noinline__ void fill_padding(uint32_t* s, int n, uint32_t base) {
   for (int i = n; i < kBlock; i++) s[i] = i >= 16 ? s[i - 16] : base;
 }
 

@@ -19,7 +19,7 @@ struct PackArgs {
   unsigned long long* counter;  // tile work counter (scratch)
   uint64_t* tile_status;        // look-back states (scratch)
   uint32_t* err;
-  uint64_t* stats = nullptr;    // set by the launcher: packed bytes and blocks of the batch
+  uint64_t* stats = nullptr;    // set by the launcher: where the kernel leaves the batch's packed bytes and blocks
   uint32_t spin_limit = 1u << 22;  // polls of each bounded wait (UTL_KNOB_SPIN_LIMIT)
 };
 
@@ -81,17 +81,21 @@ int64_t tiles_for(int64_t n_blocks);
 inline size_t pack_scratch_bytes(int64_t n_blocks) { return 16 + 8 * (size_t)tiles_for(n_blocks); }
 cudaError_t plan(const uint64_t* val_off, int n, uint64_t* bstart, cudaStream_t st);
 cudaError_t stream_offsets(const uint64_t* block_off, const uint64_t* bstart, int n, uint64_t* sbo, cudaStream_t st);
-// may_alloc false: the launch makes no allocation of any kind (the uint32
-// lane pack then skips its mapped-memory window hint).
-cudaError_t pack(bool u64, const PackArgs& a, cudaStream_t st, bool may_alloc);
+// The batched pack: first whether the batch takes two launches by the schedule
+// in force (asked once a batch: the answer may change with the packs before it)
+// and whether that needs the scratch cleared, then the launch.  may_alloc
+// false: no allocation of any kind, and no density hints (mapped memory).
+cudaError_t pack_route(bool u64, int flag, int64_t n_blocks, bool may_alloc, bool* two);
+bool pack_needs_clear(bool two, int64_t n_blocks);
+cudaError_t pack(bool u64, bool two, const PackArgs& a, cudaStream_t st, bool may_alloc);
 // utl_pack.cu: the pack in two launches, its kernels' attributes (set with the
-// other kernels' on a device's first use), the batches that take it by default,
+// other kernels' on a device's first use), the batches that take it by default
+// (mean: bytes a block of the device's last large NoPatch batch, 0: not known),
 // and whether it needs its scratch cleared.
 cudaError_t pack_two_setup();
 cudaError_t pack_two(bool u64, const PackArgs& a, cudaStream_t st);
-bool pack_by_two(bool u64, int flag, int64_t n_blocks);
+bool pack_by_two(bool u64, int flag, int64_t n_blocks, uint64_t mean);
 bool pack_two_clears(int64_t n_blocks);
-bool pack_needs_clear(bool u64, int flag, int64_t n_blocks);  // of the schedule in force
 cudaError_t unpack(bool u64, const UnpackArgs& a, cudaStream_t st);
 cudaError_t get(bool u64, const GetArgs& a, cudaStream_t st);
 cudaError_t plain_pack(bool u64, int flag, const void* vals, int n, uint8_t* out, PlainResult* res, cudaStream_t st);

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "utl_lane.cuh"
 #include "utl_launch.h"
 #include "utl_qpack.cuh"
 #include "utl_streams.cuh"
@@ -273,7 +274,13 @@ __global__ void __launch_bounds__(kThreads, U64 ? 4 : 6) write_kernel(PackArgs a
   __syncthreads();  // every warp has read the tile's plans
   if (warp == 0 && bl < a.n_blocks) {
     a.block_off[bl] = before + excl;
-    if (bl == a.n_blocks - 1) a.block_off[a.n_blocks] = before + incl;
+    if (bl == a.n_blocks - 1) {
+      a.block_off[a.n_blocks] = before + incl;
+      if (!U64 && a.stats) {  // for the next batch's route
+        a.stats[0] = before + incl;
+        a.stats[1] = (uint64_t)a.n_blocks;
+      }
+    }
   }
   const uint32_t w0 = __shfl_sync(kFull, excl, warp * 8), w1 = __shfl_sync(kFull, incl, warp * 8 + 7);
   const uint64_t g = before + w0;
@@ -381,17 +388,22 @@ static cudaError_t pack_run(const PackArgs& a, const qp::Sums& s, cudaStream_t s
   return cudaLaunchKernelEx(&c, qp::write_kernel<DELTA, U64>, a, s);
 }
 
-// Which batches take the two launches: uint64 and NoPatch ones of any size
-// (2^26 uint64 values of three shapes 903 -> 489 us, 2^27 values without
-// patching 591 -> 360 us: the one-launch pack's image holds a fraction of a
-// tile of such blocks), and all others up to kSmallBlocks blocks, where the
-// one-launch pack's warps, a tile of 32 blocks each, leave SMs idle: 2^20
+// Which batches take the two launches: uint64 ones of any size (2^26 values of
+// three shapes 903 -> 489 us), and all others up to kSmallBlocks blocks, where
+// the one-launch pack's warps, a tile of 32 blocks each, leave SMs idle: 2^20
 // outlier values 16.4 -> 13.1 us, as many postings in 128 lists 36 -> 25 us.
 // Above, the one-launch pack reads the values once: 2^22 outlier values 20.0
-// against 22.5 us, 2^28 495 against 627.
+// against 22.5 us, 2^28 495 against 627.  But its image holds a tile of blocks
+// of up to kWindow / 32 bytes each; a tile of larger ones takes several rounds.
+// Only NoPatch data has such blocks as a rule, and only then: 2^27 values under
+// NoPatch, one launch against two, in blocks of 132 bytes 168 us : 240, 196
+// bytes 192 : 259, 260 bytes 352 : 257, 438 bytes 532 : 301.  So a large NoPatch
+// batch goes by the mean block of the one before it, and by one launch while
+// that is not known.
 constexpr int64_t kSmallBlocks = 16384;
-bool pack_by_two(bool u64, int flag, int64_t n_blocks) {
-  return u64 || (flag & kNoPatch) || n_blocks <= kSmallBlocks;
+constexpr uint64_t kRoundBlock = lane::kWindow / 32;
+bool pack_by_two(bool u64, int flag, int64_t n_blocks, uint64_t mean) {
+  return u64 || n_blocks <= kSmallBlocks || ((flag & kNoPatch) && mean > kRoundBlock);
 }
 bool pack_two_clears(int64_t n_blocks) { return n_blocks > (int64_t)qp::kDirectTiles * qp::kTile; }
 
