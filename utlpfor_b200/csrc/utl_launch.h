@@ -37,6 +37,7 @@ struct UnpackArgs {
   uint32_t spin_limit = 1u << 22;  // polls of each bounded wait (UTL_KNOB_SPIN_LIMIT)
   uint64_t lane_mean = 0;  // > 0: the small-staging pipe instance leaves batches of at most this mean block length
                            // to the thread-per-block kernel launched beside it
+  int64_t quad_blocks = 0;  // unpack_auto_kernel: batches of up to so many blocks go to the quad pipeline
 };
 
 struct GetArgs {
