@@ -13,13 +13,14 @@
 // settled on its guesses; the starts are kept as bits and a second launch
 // turns them into offsets.
 //
-// A region whose chain fails (a wrong guess that was told, or a bad block)
-// leaves the whole call to the second path, which handles everything and finds
-// the first bad block: the stream is cut into partitions of kPart bytes; one thread per partition finds a
-// position where kSync consecutive headers parse and stay inside the stream
-// (a true block start lies within the first kMaxBlock bytes of every
-// partition), walks from there to the partition's end and records where its
-// chain leaves the partition.  A second pass checks, in parallel, that the
+// The first region whose chain stops at its true entry's bad block ends the
+// walk: the second launch counts the blocks before it.  A region that told a
+// wrong exit leaves the whole call to the second path, which handles
+// everything: the stream is cut into partitions of kPart bytes; one thread per
+// partition finds a position where kSync consecutive headers parse and stay
+// inside the stream (a true block start lies within the first kMaxBlock bytes
+// of every partition), walks from there to the partition's end and records
+// where its chain leaves the partition.  A second pass checks, in parallel, that the
 // chain entering each partition (the previous partition's exit) meets that
 // partition's chain -- two chains that share one position share all later
 // ones -- and derives the partition's true block count.  Partitions whose
@@ -307,10 +308,11 @@ __global__ void __launch_bounds__(kThreads) write_kernel(const uint8_t* p, uint6
 // ---- the first path ----
 // Bound by the latency of guessing and walking (dependent shared-memory loads
 // and byte arithmetic) with 24 warps on an SM, not by its one read of the
-// stream: 2^26 outlier values under NoFOR (75 MB, 524 289 blocks) take 46 us
-// here, 8 us in the second launch and 66 us for the whole call, against 397 us
-// by the second path (a thread per 8 KB on global memory, and five round trips
-// with the host).
+// stream: 2^26 outlier values under NoFOR (75 MB, 2331 regions, 524 289 blocks)
+// take 34 us here, 8 us in the second launch and 60 us for the whole call,
+// against 397 us by the second path (a thread per 8 KB on global memory, and
+// five round trips with the host).  A bad block half way: 44 us for 2^25 values
+// (343 us when it was left to the second path as well, 309 by that alone).
 // A team of four threads has 1008 bytes.  Finding a start takes about a block
 // length of places to look at, so four threads share it; walking is serial
 // and one does it.  252 words from team to team put the eight teams of a warp,
@@ -325,15 +327,27 @@ constexpr int kAhead = 32;                // staged bytes past the region (heade
 static_assert(kRegion % 16 == 0, "regions keep the stream's alignment");
 constexpr uint32_t kDrainPolls = 1u << 22;  // for a copy that must land before the CTA ends, whatever the knob says
 
-// Result of the first path: the block count, and whether it holds.
-struct FastResult {
+// Result of the first path: the block count, or the status and the index of
+// the first bad block; open: neither is known.
+struct __align__(16) FastResult {
   int64_t blocks;
-  int32_t bad;
-  int32_t pad;
+  int32_t status;
+  int32_t open;
 };
+// The first region that failed, and how: all regions before it are right, so
+// its own entry is the stream's, and a chain that stops there stops at the
+// stream's first bad block.  A region without an entry (the one before it
+// failed, or a wait ran out) or whose exit is not what it told says nothing.
+// Held as ~key, so that zero is none and the maximum the first region.
 struct FastCtl {
-  uint32_t ticket, bad, pad[2];
+  uint32_t ticket, pad;
+  unsigned long long worst;
 };
+constexpr uint32_t kOpen = 0xFFFF;  // in place of the bad block's position
+static_assert(kRegion < 0xFFFF, "positions in 16 bits");
+__device__ __forceinline__ void fail_region(FastCtl* ctl, int32_t r, uint32_t pos) {
+  atomicMax(&ctl->worst, ~(((unsigned long long)(uint32_t)r << 16) | pos));
+}
 
 // What the two launches share: block counts of the regions, of their groups
 // of 32 and of 1024, and the block starts of each region as bits (a word row
@@ -429,7 +443,7 @@ __global__ void __launch_bounds__(kRT) index_starts_kernel(const uint8_t* p, uin
   __shared__ __align__(16) uint32_t buf[(16 + kRegion + kAhead + 16) / 4];
   __shared__ uint32_t bits[kTeams][kBitWords | 1];  // block starts in each team's bytes
   __shared__ int X[kTeams];  // where each team's chain leaves its bytes (-1: not known, -2: it failed)
-  __shared__ int s_region, s_entry, s_from;
+  __shared__ int s_region, s_entry, s_from, s_bad;
   __shared__ uint32_t s_total;
   __shared__ uint64_t bar;
   const int k = threadIdx.x, lane = k & 31;
@@ -438,6 +452,7 @@ __global__ void __launch_bounds__(kRT) index_starts_kernel(const uint8_t* p, uin
     tma::mbar_init_fence();
     s_region = (int)atomicAdd(&tab.ctl->ticket, 1u);
     s_total = 0;
+    s_bad = (int)kOpen;
   }
   __syncthreads();
   const int32_t r = s_region;
@@ -468,12 +483,11 @@ __global__ void __launch_bounds__(kRT) index_starts_kernel(const uint8_t* p, uin
     // to land before the CTA's shared memory goes to another one.
     if (k == 0) {
       *(volatile int64_t*)&tab.exits[r] = -1;
-      atomicOr(&tab.ctl->bad, 1u);
+      fail_region(tab.ctl, r, kOpen);
     }
     tma::mbar_wait(&bar, 0, kDrainPolls);
     return;
   }
-  bool failed = false;
 
   // a start per team, guessed: the four threads look at alternate pairs of words
   const int team = k / kTeam, c4 = k % kTeam;
@@ -529,12 +543,16 @@ __global__ void __launch_bounds__(kRT) index_starts_kernel(const uint8_t* p, uin
   }
   __syncwarp();
   if (k == 0) s_entry = t;
-  // walk from t through the team's bytes (its first thread)
+  // walk from t through the team's bytes (its first thread); -2 at a bad block
+  int stuck = 0;
   const auto walk = [&]() {
     int x = t;
     while (x < own_end && x < s.end) {
       const int n = region_length(s, x);
-      if (n == 0) return -2;
+      if (n == 0) {
+        stuck = x;
+        return -2;
+      }
       const int b = x - own;
       bits[team][b >> 5] |= 1u << (b & 31);
       x += n;
@@ -586,8 +604,9 @@ __global__ void __launch_bounds__(kRT) index_starts_kernel(const uint8_t* p, uin
   // and the teams settle again if it differs; the exit has to stay what was
   // told.  (exits: position + 1; 0 = not yet,
   // -1 = failed.)
-  bool told = leave >= 0;
-  if (k == 0 && told) *(volatile int64_t*)&tab.exits[r] = start + leave + 1;
+  const int first_leave = leave;
+  bool entered = true;
+  if (k == 0 && leave >= 0) *(volatile int64_t*)&tab.exits[r] = start + leave + 1;
   if (r > 0) {
     if (k == 0) {
       int64_t e = 0;
@@ -599,20 +618,20 @@ __global__ void __launch_bounds__(kRT) index_starts_kernel(const uint8_t* p, uin
     }
     __syncthreads();
     const int from = s_from;
+    entered = from >= 0;
     if (from != s_entry) {
       __syncthreads();
       if (k == 0) s_entry = from;
       __syncthreads();
-      const int again = from < 0 ? -2 : settle();
-      if (again < 0 || (told && again != leave)) failed = true;
-      leave = again;
+      leave = entered ? settle() : -2;
     }
-  } else if (!told) {
-    failed = true;
   }
-  if (k == 0 && !told) *(volatile int64_t*)&tab.exits[r] = failed ? -1 : start + leave + 1;
-
-  if (r == n_regions - 1 && start + leave != (int64_t)len) failed = true;
+  if (k == 0 && first_leave < 0) *(volatile int64_t*)&tab.exits[r] = leave >= 0 ? start + leave + 1 : -1;
+  // The first team of a chain that stopped is the one that met the bad block
+  // (the others only took that over).
+  if (entered && leave < 0 && first && X[team] == -2 && (team == 0 || X[team - 1] != -2)) s_bad = stuck;
+  const bool failed = leave < 0 || (first_leave >= 0 && leave != first_leave) ||
+                      (r == n_regions - 1 && start + leave != (int64_t)len);
 
   // the starts and their counts, for the second launch
   int c = 0;
@@ -626,21 +645,33 @@ __global__ void __launch_bounds__(kRT) index_starts_kernel(const uint8_t* p, uin
   }
   c = (int)__reduce_add_sync(kFull, (unsigned)c);
   if (lane == 0) atomicAdd(&s_total, (uint32_t)c);
-  failed = __syncthreads_or(failed);
+  __syncthreads();
   if (k == 0) {
     tab.one[r] = s_total;
     atomicAdd(&tab.g32[r >> 5], s_total);
     atomicAdd(&tab.g1024[r >> 10], (unsigned long long)s_total);
-    if (failed) atomicOr(&tab.ctl->bad, 1u);
+    if (failed) fail_region(tab.ctl, r, (uint32_t)s_bad);
   }
+}
+
+// The stream's first bad block, at place bad of region r, by the thread whose
+// eight words its start would be in: its index is the count of the starts
+// before it, at of them in the words before.
+__device__ __noinline__ void report_bad(const uint8_t* p, uint64_t len, int32_t r, int bad, int64_t at,
+                                        const uint32_t* words, FastResult* result) {
+  const int places = bad % kSub & 255;  // of these words before it
+  for (int i = 0; 32 * i < places; i++)
+    at += __popc(places - 32 * i >= 32 ? words[i] : words[i] & ((1u << (places - 32 * i)) - 1u));
+  uint64_t n;
+  const int status = block_length_at(p, len, (uint64_t)r * kRegion + (uint64_t)bad, &n);
+  *result = FastResult{at, status, status == kOK ? 1 : 0};
 }
 
 // The offsets of a region's blocks from its starts: a thread per eight words
 // of bits, after the blocks before the region.  (In the first launch a region
-// would have to wait for all before it: 65 us against 43 + 5 here for 2331
-// regions.)
-__global__ void __launch_bounds__(kRT) index_write_kernel(uint64_t len, int32_t n_regions, RegionTables tab,
-                                                          uint64_t* block_off, int64_t max_blocks,
+// would have to wait for all before it, which cost half as much again.)
+__global__ void __launch_bounds__(kRT) index_write_kernel(const uint8_t* p, uint64_t len, int32_t n_regions,
+                                                          RegionTables tab, uint64_t* block_off, int64_t max_blocks,
                                                           FastResult* result) {
   static_assert(kTeams * kBitWords == 8 * kRT, "eight words a thread");
   __shared__ int wsum[kRT / 32];
@@ -648,6 +679,7 @@ __global__ void __launch_bounds__(kRT) index_write_kernel(uint64_t len, int32_t 
   const int32_t r = blockIdx.x;
   const uint4* in = (const uint4*)(tab.bits + (size_t)r * (kTeams * kBitWords)) + 2 * k;
   const uint4 A = in[0], B = in[1];
+  const unsigned long long worst = ~__ldg(&tab.ctl->worst);
   const int r32 = r & ~31, r1024 = r & ~1023;
   uint64_t sum = (r32 + lane < r ? tab.one[r32 + lane] : 0u);
   if (r1024 + 32 * lane < r32) sum += tab.g32[(r1024 >> 5) + lane];
@@ -671,8 +703,11 @@ __global__ void __launch_bounds__(kRT) index_write_kernel(uint64_t len, int32_t 
       if (at < max_blocks) block_off[at] = first + (uint64_t)(32 * i + __ffs(b) - 1);
   if (r == n_regions - 1 && k == kRT - 1) {
     if (at <= max_blocks) block_off[at] = len;
-    result->blocks = at;
-    result->bad = tab.ctl->bad ? 1 : 0;
+    if (worst == ~0ull || (worst & 0xFFFFu) == kOpen) *result = FastResult{at, kOK, worst == ~0ull ? 0 : 1};
+  }
+  if ((uint32_t)(worst >> 16) == (uint32_t)r && (worst & 0xFFFFu) != kOpen && worst != ~0ull) {
+    const int bad = (int)(worst & 0xFFFFu);
+    if (k == kTeam * (bad / kSub) + (bad % kSub >> 8)) report_bad(p, len, r, bad, at - c, (const uint32_t*)in, result);
   }
 }
 
@@ -711,14 +746,15 @@ int index_stream(const uint8_t* p, uint64_t len, uint64_t* block_off, int64_t ma
     const RegionTables tab = tables(scratch, n_regions);
     if ((*cerr = cudaMemsetAsync(scratch, 0, tables_zeroed(n_regions), st)) != cudaSuccess) return -1;
     index_starts_kernel<<<(unsigned)n_regions, kRT, 0, st>>>(p, len, (int32_t)n_regions, tab, spin_limit());
-    index_write_kernel<<<(unsigned)n_regions, kRT, 0, st>>>(len, (int32_t)n_regions, tab, block_off, max_blocks,
+    index_write_kernel<<<(unsigned)n_regions, kRT, 0, st>>>(p, len, (int32_t)n_regions, tab, block_off, max_blocks,
                                                             (FastResult*)res_d);
     note_launch(2);
     if ((*cerr = cudaGetLastError()) != cudaSuccess) return -1;
     if ((*cerr = cudaStreamSynchronize(st)) != cudaSuccess) return -1;
     const FastResult f = *(const FastResult*)res_h;
-    if (!f.bad) {
+    if (!f.open) {
       *n_blocks = f.blocks;
+      if (f.status != kOK) return f.status;
       return f.blocks > max_blocks ? kErrCapacity : kOK;
     }
   }
