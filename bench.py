@@ -657,7 +657,7 @@ def main():
         codec.pack(values)
         torch.cuda.synchronize()
         two = L.utl_launch_count() - launches0 == 2
-        kname = "plan_kernel+write_kernel" if two else \
+        kname = "pack_plan_kernel+pack_write_kernel" if two else \
             ("pack_kernel" if sched == 0 else "pack_lane_kernel") if is64 else \
             pack_names.get(sched, "pack_lane_kernel")
     elif is64:

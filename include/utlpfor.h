@@ -172,7 +172,7 @@ UTL_API int utl_batch_plan(const uint64_t *d_val_off, int n_streams,
                    uint64_t *d_block_start, void *stream);
 
 /* Device scratch the pack needs for n_blocks blocks (tile states of the
- * single-pass offset scan). */
+ * single-pass offset scan, or the length sums of the two-launch pack). */
 UTL_API size_t utl_pack_scratch_bytes(int64_t n_blocks);
 
 /* Pack every block of every stream.  d_block_off (n_blocks+1) receives each
@@ -201,7 +201,7 @@ UTL_API int utl_pack_batch_u64(uint8_t flag, const uint64_t *d_values,
  * memory budget and hand out no allocation rights (a Go process calling
  * through cgo that manages every device byte itself).  It has no counterpart in the reference (the Go library
  * never touches device memory).  Same arguments as utl_pack_batch_u32
- * without the scratch: the look-back tile states live in a 2 MiB array
+ * without the scratch: what the pack keeps between tiles lives in a 2 MiB array
  * built into the library, which every GPU that loads the library keeps
  * until the process exits.  Batches above
  * utl_pack_batch_u32_noalloc_max_blocks() blocks (about 4.2 million, i.e.

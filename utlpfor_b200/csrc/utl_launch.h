@@ -16,8 +16,8 @@ struct PackArgs {
   uint8_t* out;
   uint64_t out_cap;
   uint64_t* block_off;
-  unsigned long long* counter;  // tile work counter (scratch)
-  uint64_t* tile_status;        // look-back states (scratch)
+  unsigned long long* counter;  // the scratch: tile work counter
+  uint64_t* tile_status;        // and look-back states (one launch), or all of it the length sums (two)
   uint32_t* err;
   uint64_t* stats = nullptr;    // set by the launcher: where the kernel leaves the batch's packed bytes and blocks
   uint32_t spin_limit = 1u << 22;  // polls of each bounded wait (UTL_KNOB_SPIN_LIMIT)
@@ -78,7 +78,11 @@ namespace launch {
 size_t pack_smem(bool u64);
 size_t unpack_smem(bool u64);
 int64_t tiles_for(int64_t n_blocks);
-// scratch layout of the pack: [0,8) work counter, [16, 16+8*tiles) tile states
+// Scratch of the pack, a tile being 16 blocks here.  In one launch: [0,8) work
+// counter, [16, 16 + 8 * tiles) tile states, all of it zero at the start.  In two
+// launches: the packed bytes per 1024 * 32, 32 and 32 * 32 blocks (utl_pack.cu,
+// Sums; at most 4 1/8 bytes per 32 blocks), zero at the start only where there
+// are groups (pack_two_clears).
 inline size_t pack_scratch_bytes(int64_t n_blocks) { return 16 + 8 * (size_t)tiles_for(n_blocks); }
 cudaError_t plan(const uint64_t* val_off, int n, uint64_t* bstart, cudaStream_t st);
 cudaError_t stream_offsets(const uint64_t* block_off, const uint64_t* bstart, int n, uint64_t* sbo, cudaStream_t st);

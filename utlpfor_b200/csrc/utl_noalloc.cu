@@ -6,8 +6,8 @@
 // memory budget up front (a Go process calling through cgo that manages
 // every device byte itself).
 // utl_pack_batch_u32_noalloc serves them: the caller passes only inputs and
-// outputs, and the look-back tile states live in the fixed-size array
-// below instead of caller-provided or library-allocated scratch.
+// outputs, and what the pack keeps between its tiles lives in the fixed-size
+// array below instead of caller-provided or library-allocated scratch.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -18,9 +18,8 @@
 
 namespace utl {
 
-// Scratch of the no-allocation pack (2 MiB): the tile work counter and one
-// 8-byte look-back state per tile, laid out as utl_pack_scratch_bytes
-// describes.  Every GPU that loads this library holds these bytes until
+// Scratch of the no-allocation pack (2 MiB), of either layout that
+// launch::pack_scratch_bytes describes.  Every GPU that loads this library holds these bytes until
 // the process exits.  In host code the name is only a host-side stand-in
 // for the device array; its device address comes from cudaGetSymbolAddress.
 constexpr size_t kNoAllocScratchBytes = (size_t)2 << 20;
@@ -70,8 +69,8 @@ extern "C" int utl_pack_batch_u32_noalloc(uint8_t flag, const uint32_t* d_values
     }
     scratch = g_addr[dev];
   }
-  // The array keeps the previous call's contents; the pack clears the
-  // counter and tile states it uses on `stream` before its kernel runs.
+  // The array keeps the previous call's contents; the pack clears on `stream`,
+  // before its first kernel runs, what has to start at zero.
   // may_alloc = false: the launch takes no allocating step at all (the
   // uint32 pack's mapped-memory window hint is skipped).
   return pack_batch_device(false, false, flag, d_values, d_val_off, d_block_start, n_streams, n_blocks, d_out, out_cap,

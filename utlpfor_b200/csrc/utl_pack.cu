@@ -1,8 +1,8 @@
 // utl_pack.cu -- the batched pack in two launches (utl_qpack.cuh).
 //
-// The first (plan_kernel) reads the values and decides every block: its plan
+// The first (pack_plan_kernel) reads the values and decides every block: its plan
 // goes into the block's entry of the offset table, the packed lengths are
-// summed per 32, 1024 and 32768 blocks.  The second (write_kernel) knows the
+// summed per 32, 1024 and 32768 blocks.  The second (pack_write_kernel) knows the
 // byte offset of its blocks from those sums, reads the values again, writes
 // the blocks into an image with the output's alignment and sends it out by a
 // bulk store.  No block waits for another, neither kernel holds values in
@@ -42,6 +42,9 @@ struct Sums {
   unsigned long long* g1024;  // null: no groups
 };
 // In the pack's scratch: 4 1/8 bytes per 32 blocks, of its 16.
+inline size_t sums_bytes(int64_t n_tiles) {
+  return 8 * (size_t)((n_tiles + 1023) / 1024) + 4 * (size_t)n_tiles + 4 * (size_t)((n_tiles + 31) / 32);
+}
 inline Sums sums_in(void* scratch, int64_t n_tiles) {
   Sums s;
   s.g1024 = (unsigned long long*)scratch;
@@ -185,7 +188,7 @@ __device__ __forceinline__ Shape64 shape64(const uint32_t (&x)[8][4], const uint
 constexpr int kFor64Bit = 2 * kPlanBits, kTwoBit = kFor64Bit + 1;
 
 template <bool DELTA, bool U64>
-__global__ void __launch_bounds__(kThreads, U64 ? 4 : 6) plan_kernel(PackArgs a, Sums sums) {
+__global__ void __launch_bounds__(kThreads, U64 ? 4 : 6) pack_plan_kernel(PackArgs a, Sums sums) {
   __shared__ uint32_t s_len;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = lane >> 2, j = lane & 3;
   const int64_t t = blockIdx.x, b0 = t * kTile + warp * 8, b = b0 + q;
@@ -236,7 +239,7 @@ struct __align__(16) WriteSmem {
 };
 
 template <bool DELTA, bool U64>
-__global__ void __launch_bounds__(kThreads, U64 ? 4 : 6) write_kernel(PackArgs a, Sums sums) {
+__global__ void __launch_bounds__(kThreads, U64 ? 4 : 6) pack_write_kernel(PackArgs a, Sums sums) {
   extern __shared__ uint4 smem4[];
   WriteSmem<U64>& S = *(WriteSmem<U64>*)smem4;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = lane >> 2, j = lane & 3;
@@ -358,7 +361,7 @@ namespace launch {
 
 template <bool DELTA, bool U64>
 static cudaError_t pack_attr() {
-  const auto k = qp::write_kernel<DELTA, U64>;
+  const auto k = qp::pack_write_kernel<DELTA, U64>;
   const cudaError_t e =
       cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(qp::WriteSmem<U64>));
   if (e == cudaSuccess) cudaFuncSetAttribute((const void*)k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -374,7 +377,7 @@ cudaError_t pack_two_setup() {
 
 template <bool DELTA, bool U64>
 static cudaError_t pack_run(const PackArgs& a, const qp::Sums& s, cudaStream_t st) {
-  qp::plan_kernel<DELTA, U64><<<(unsigned)a.n_tiles, qp::kThreads, 0, st>>>(a, s);
+  qp::pack_plan_kernel<DELTA, U64><<<(unsigned)a.n_tiles, qp::kThreads, 0, st>>>(a, s);
   cudaLaunchConfig_t c = {};
   cudaLaunchAttribute early;
   early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -385,7 +388,7 @@ static cudaError_t pack_run(const PackArgs& a, const qp::Sums& s, cudaStream_t s
   c.stream = st;
   c.attrs = &early;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, qp::write_kernel<DELTA, U64>, a, s);
+  return cudaLaunchKernelEx(&c, qp::pack_write_kernel<DELTA, U64>, a, s);
 }
 
 // Which batches take the two launches: uint64 ones of any size (2^26 values of
@@ -411,7 +414,7 @@ cudaError_t pack_two(bool u64, const PackArgs& a_in, cudaStream_t st) {
   cudaError_t e;
   PackArgs a = a_in;
   a.n_tiles = (a.n_blocks + qp::kTile - 1) / qp::kTile;
-  if (a.n_tiles > INT32_MAX) return cudaErrorInvalidValue;
+  if (a.n_tiles > INT32_MAX || qp::sums_bytes(a.n_tiles) > pack_scratch_bytes(a.n_blocks)) return cudaErrorInvalidValue;
   const qp::Sums s = qp::sums_in(a.counter, a.n_tiles);
   const bool d = (a.flag & kDelta) != 0;
   if (u64) e = d ? pack_run<true, true>(a, s, st) : pack_run<false, true>(a, s, st);
