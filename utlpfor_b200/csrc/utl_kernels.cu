@@ -1177,18 +1177,20 @@ __global__ void __launch_bounds__(32 * W, 16 / W) unpack_lane_kernel(UnpackArgs 
 constexpr size_t kAutoSmem = sizeof(LaneUnpackSmem<1, kLUStage1, 4>) > sizeof(QuadPipeSmem<kPStageWide, 2>)
                                  ? sizeof(LaneUnpackSmem<1, kLUStage1, 4>)
                                  : sizeof(QuadPipeSmem<kPStageWide, 2>);
-// Up to quad_blocks blocks, one group of eight for every resident warp and a
-// second one for a fifth of them, the quad pipeline is taken whatever the mean
-// length: a warp's 32 blocks one after the other leave most of the SMs idle.
+// Up to kQuadBlocks blocks, one group of eight for each of a B200's resident
+// warps and a second one for a fifth of them, the quad pipeline is taken
+// whatever the mean length: a warp's 32 blocks one after the other leave most of the SMs idle.
 // Thread path against quads, one stream and 400 ragged ones, outlier values:
 // 8192 blocks 9.7 : 4.6 and 17.6 : 9.6 us, 22 000 blocks 12.0 : 10.5 and 17.6 :
 // 14.5.  Beyond, it depends on how the groups and tiles fall on the warps:
 // 26 000 blocks 12.0 : 11.0 but 15.2 : 17.3, 37 000 blocks 11.2 : 12.3 and
-// 16.1 : 19.5 (postings 12.0 : 10.6 and 20.2 : 20.9).
+// 16.1 : 19.5 (postings 12.0 : 10.6 and 20.2 : 20.9).  (Given by the launch
+// instead of as a constant, the thread path takes 0.6% longer on the lists.)
+constexpr int64_t kQuadBlocks = 148 * 16 * 8 * 6 / 5;
 __global__ void __launch_bounds__(kQThreads, 4) unpack_auto_kernel(UnpackArgs a) {
   extern __shared__ uint4 smem4[];
   const uint64_t span = a.block_off[a.n_blocks] - a.block_off[0];
-  if (a.n_blocks > a.quad_blocks && span <= kWideMean * (uint64_t)a.n_blocks) lane_body<1, kLUStage1, 4>(a, smem4);
+  if (a.n_blocks > kQuadBlocks && span <= kWideMean * (uint64_t)a.n_blocks) lane_body<1, kLUStage1, 4>(a, smem4);
   else pipe_body<kPStageWide, false, 2>(a, smem4);
 }
 
@@ -2865,12 +2867,10 @@ static cudaError_t unpack_pipe(const UnpackArgs& a, cudaStream_t st, int ctas) {
   note_launch(1);
   return cudaGetLastError();
 }
-static cudaError_t unpack_auto(const UnpackArgs& a_in, cudaStream_t st, int ctas) {
+static cudaError_t unpack_auto(const UnpackArgs& a, cudaStream_t st, int ctas) {
   // persistent over the finer of the two paths' work items (8-block groups)
-  UnpackArgs a = a_in;
   const int64_t groups = (a.n_blocks + 7) / 8;
   int64_t grid = (int64_t)num_sms() * unpack_ctas(ctas);
-  a.quad_blocks = grid * kQWarps * 8 * 6 / 5;
   const int64_t need = (groups + kQWarps - 1) / kQWarps;
   if (grid > need) grid = need;
   unpack_auto_kernel<<<(unsigned)grid, kQThreads, kAutoSmem, st>>>(a);
@@ -3018,6 +3018,7 @@ static int pick_window(PackArgs& a, bool may_alloc, DevCfg& c, uint64_t small_bl
   const int pair = stats_pair(a.flag);
   uint64_t mean = stats_mean(c, pair);
   if (mean == 0) mean = stats_mean(c, 2 - pair);
+  static_assert(kRoundBlock == lane::kWindow / 32, "a tile of 32 blocks in the large window");
   return (mean > 0 && mean <= small_block) ? 1 : 0;
 }
 

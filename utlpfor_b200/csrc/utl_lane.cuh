@@ -162,7 +162,7 @@ __device__ __forceinline__ uint32_t work_at(const uint32_t* s, int pos, uint32_t
 // is set so that its work values are zero, as the reference leaves them
 // (scalar.go:34-40, delta.go:23-48): base in row 0, the lane's value one
 // row up below it.
-static __device__ __noinline__ void fill_padding(uint32_t* s, int n, uint32_t base) {
+__device__ __noinline__ void fill_padding(uint32_t* s, int n, uint32_t base) {
   for (int i = n; i < kBlock; i++) s[i] = i >= 16 ? s[i - 16] : base;
 }
 

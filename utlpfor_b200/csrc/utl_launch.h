@@ -37,7 +37,6 @@ struct UnpackArgs {
   uint32_t spin_limit = 1u << 22;  // polls of each bounded wait (UTL_KNOB_SPIN_LIMIT)
   uint64_t lane_mean = 0;  // > 0: the small-staging pipe instance leaves batches of at most this mean block length
                            // to the thread-per-block kernel launched beside it
-  int64_t quad_blocks = 0;  // unpack_auto_kernel: batches of up to so many blocks go to the quad pipeline
 };
 
 struct GetArgs {
@@ -101,6 +100,7 @@ cudaError_t pack_two_setup();
 cudaError_t pack_two(bool u64, const PackArgs& a, cudaStream_t st);
 bool pack_by_two(bool u64, int flag, int64_t n_blocks, uint64_t mean);
 bool pack_two_clears(int64_t n_blocks);
+constexpr uint64_t kRoundBlock = 224;  // bytes a block up to which the one-launch pack's image holds a whole tile
 cudaError_t unpack(bool u64, const UnpackArgs& a, cudaStream_t st);
 cudaError_t get(bool u64, const GetArgs& a, cudaStream_t st);
 cudaError_t plain_pack(bool u64, int flag, const void* vals, int n, uint8_t* out, PlainResult* res, cudaStream_t st);

@@ -19,7 +19,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "utl_lane.cuh"
 #include "utl_launch.h"
 #include "utl_qpack.cuh"
 #include "utl_streams.cuh"
@@ -397,14 +396,13 @@ static cudaError_t pack_run(const PackArgs& a, const qp::Sums& s, cudaStream_t s
 // outlier values 16.4 -> 13.1 us, as many postings in 128 lists 36 -> 25 us.
 // Above, the one-launch pack reads the values once: 2^22 outlier values 20.0
 // against 22.5 us, 2^28 495 against 627.  But its image holds a tile of blocks
-// of up to kWindow / 32 bytes each; a tile of larger ones takes several rounds.
+// of up to kRoundBlock bytes each; a tile of larger ones takes several rounds.
 // Only NoPatch data has such blocks as a rule, and only then: 2^27 values under
 // NoPatch, one launch against two, in blocks of 132 bytes 168 us : 240, 196
 // bytes 192 : 259, 260 bytes 352 : 257, 438 bytes 532 : 301.  So a large NoPatch
 // batch goes by the mean block of the one before it, and by one launch while
 // that is not known.
 constexpr int64_t kSmallBlocks = 16384;
-constexpr uint64_t kRoundBlock = lane::kWindow / 32;
 bool pack_by_two(bool u64, int flag, int64_t n_blocks, uint64_t mean) {
   return u64 || n_blocks <= kSmallBlocks || ((flag & kNoPatch) && mean > kRoundBlock);
 }
