@@ -12,8 +12,9 @@
 //
 // Measured on 2^26 uint64 values of three shapes: 489 us (903 in one launch),
 // of which the first launch is about 130 (its read of 537 MB takes 82 at the
-// copy rate) and the second the rest, bound by its 2100 instructions per eight
-// blocks at 14 warps on an SM.  One warp writing the exceptions of the tile's
+// copy rate) and the second the rest: at 14 warps on an SM it issues 35% of the
+// time and waits for loads and for shared memory, about two cycles per issue
+// each.  One warp writing the exceptions of the tile's
 // 32 blocks, a lane each, executes fewer instructions but leaves three warps
 // at a barrier: 577 us, and 695 against 627 on 2^28 outlier values.
 #include <cuda_runtime.h>
@@ -394,6 +395,9 @@ static cudaError_t pack_run(const PackArgs& a, const qp::Sums& s, cudaStream_t s
 // three shapes 903 -> 489 us), and all others up to kSmallBlocks blocks, where
 // the one-launch pack's warps, a tile of 32 blocks each, leave SMs idle: 2^20
 // outlier values 16.4 -> 13.1 us, as many postings in 128 lists 36 -> 25 us.
+// (The host pays for the second launch: 2^12 aligned values issued back to back
+// by one thread 10.3 -> 11.4 us, where the call alone takes 22.9 -> 19.6 us and a
+// graph of them 10.4 -> 4.3 us each.)
 // Above, the one-launch pack reads the values once: 2^22 outlier values 20.0
 // against 22.5 us, 2^28 495 against 627.  But its image holds a tile of blocks
 // of up to kRoundBlock bytes each; a tile of larger ones takes several rounds.

@@ -38,7 +38,7 @@ TUNED = os.path.join(HERE, "tuned")
 # unpack staging size stay chosen per batch (window 0, unpack schedules 1,
 # 4 and 8 pick by block density), so a setting tuned on one workload cannot
 # slow down a batch of much larger blocks.
-PACK_SHAPES = [(3, 0), (2, 0), (0, 0)]  # (schedule, window); 3 is 1 on the swept batch
+PACK_SHAPES = [(3, 0), (2, 0), (0, 0)]  # (schedule, window); 3 is 1 on a swept batch of more than 2^21 values
 PACK_CAPS = [0, 16, 12, 8]
 UNPACK_SCHEDULES = [8, 1, 4, 0]
 UNPACK_CAPS = [0, 4, 3, 2]
