@@ -190,9 +190,10 @@ __global__ void __launch_bounds__(kThreads) check_kernel(const uint8_t* p, uint6
     bool ok = false;
     int64_t tc = 0;
     if (x >= 0 && r.exit >= 0) {
-      if (x >= end) {  // only at the stream's end (partitions are longer than any block)
-        ok = true;
-        tc = 0;
+      if (x >= end) {
+        // no block starts here; the partition's own chain is not the stream's,
+        // and where it leads to must not enter the next one
+        ok = end == (int64_t)len;
       } else if (y >= 0) {
         int64_t hx, hy;
         if (meet(p, len, x, y, end, &hx, &hy)) {  // the chains share every block from the meeting on
@@ -240,13 +241,7 @@ __global__ void fixup_kernel(const uint8_t* p, uint64_t len, int64_t n_parts, Pa
     if (k >= n_parts) return;
     Part& q = parts[k];
     const int64_t nend = min((int64_t)len, k * kPart + kPart);
-    if (e >= nend) {
-      q.tcount = 0;
-      q.exit = e;
-      q.ok = 1;
-      return;
-    }
-    if (q.entry >= 0 && q.exit >= 0) {
+    if (e < nend && q.entry >= 0 && q.exit >= 0) {  // a block that spans it leaves no meeting there
       int64_t hx, hy;
       if (meet(p, len, e, q.entry, nend, &hx, &hy)) {
         q.tcount = hx + q.count - hy;
